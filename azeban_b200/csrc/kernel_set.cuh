@@ -147,8 +147,13 @@ template <> struct PadStateTile<float, 768> {
   static constexpr int NC = 16, NT = 192, MINB = 2;
 };
 
+// Allows a kernel `bytes` of dynamic shared memory.  The 48 KB that need no asking count
+// its static shared memory too (the last pass at L = 512 in FP64 takes 48 KB and a step
+// size beside them).
 template <typename K> inline cudaError_t set_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  cudaFuncAttributes f;
+  const cudaError_t ce = cudaFuncGetAttributes(&f, kernel);
+  if (ce != cudaSuccess || f.sharedSizeBytes + bytes <= 48 * 1024) return ce;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
 }
 
