@@ -73,7 +73,7 @@ struct ColArgs {
 // Entry of a column pass: false if the member (blockIdx.z) is to be skipped.
 // The values that other blocks read here (time, t_end) are not written here.
 __device__ __forceinline__ bool pass_enter(const ColArgs& a) {
-  pdl_enter();
+  if (a.pdl) pdl_enter();
   if (a.ctrl == nullptr) return true;
   Ctrl* c = a.ctrl + blockIdx.z;
   const bool skip = a.begin == BEGIN_NONE ? c->skip != 0 : a.begin == BEGIN_SIM ? !(c->time < c->t_end) : false;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kProducts<3, L> * NCM * Plan<L, V>::TPL,
   C* tw = reinterpret_cast<C*>(az_smem);
   C* sm = tw + L;
   const int member = blockIdx.y;
-  pdl_enter();
+  if (a.pdl) pdl_enter();
   if (a.ctrl != nullptr && a.ctrl[member].skip) return;
   const int tid = threadIdx.x;
   const int tile = blockIdx.x;

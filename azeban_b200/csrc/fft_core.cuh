@@ -27,8 +27,9 @@ namespace azb {
 
 // Programmatic dependent launch: lets the next kernel of the stream start its
 // blocks while this one's last ones run, and waits until the kernels before
-// this one are complete and their writes visible.  Every pass kernel calls both
-// before its first access to global memory (harmless in a plain launch).
+// this one are complete and their writes visible.  A pass kernel that was launched
+// so (pdl of its arguments) calls it before its first access to global memory; in the
+// others it would only cost: 29296 fields of 16^2 transformed in 99 instead of 70 us.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");

@@ -157,16 +157,17 @@ template <typename K> inline cudaError_t set_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
 }
 
-// Fewer than two CTAs for each of the 148 SMs: a launch bound by latency.
-inline bool few_ctas(long long n) { return n < 2 * 148; }
-
-// Launches a pass kernel.  pdl: it may start before the kernel in front of it on
-// the stream has ended (it waits for that itself, pdl_enter); used for small
-// launches only.  A large one that starts on SMs still set up for the kernel in
-// front keeps that kernel's split of shared memory and L1, and with it fewer
-// CTAs per SM, to its end (a 512^3 FP32 step took 43.5 ms instead of 34.7).
-template <typename K, typename... A>
-inline cudaError_t launch_pass(K k, dim3 g, int nt, size_t smem, cudaStream_t st, int pdl, const A&... a) {
+// Launches a pass kernel.  a.pdl on entry: it may start before the kernel in front of
+// it on the stream has ended (it waits for that itself, pdl_enter); done for launches of
+// at most one CTA for every two of the 148 SMs, and a.pdl then tells the kernel whether
+// it was.  The CTAs of an early start go where room is first, several to an SM beside
+// idle ones, and to SMs still split between shared memory and L1 for the kernel in
+// front: steps (us; limit of 74 CTAs, 148, 296, none early) 2-D M = 768 FP32 58, 65, 65,
+// 58; M = 512 N = 298 FP32 90, 94, 123, 90; M = 48 N = 32 FP64 35, 35, 35, 37; 3-D
+// M = 48 N = 26 FP64 74, 74, 88, 74; all launches early: a 512^3 FP32 step 43500 instead of
+// 34700.
+template <typename K, typename A, typename... R>
+inline cudaError_t launch_pass(K k, dim3 g, int nt, size_t smem, cudaStream_t st, A a, const R&... rest) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = g;
   cfg.blockDim = dim3(unsigned(nt));
@@ -176,8 +177,9 @@ inline cudaError_t launch_pass(K k, dim3 g, int nt, size_t smem, cudaStream_t st
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = pdl && few_ctas((long long)g.x * g.y * g.z) ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k, a...);
+  a.pdl = a.pdl && (long long)g.x * g.y * g.z <= 148 / 2 ? 1 : 0;
+  cfg.numAttrs = unsigned(a.pdl);
+  return cudaLaunchKernelEx(&cfg, k, a, rest...);
 }
 
 template <typename T, int L, int V> struct LaunchV {
@@ -194,7 +196,7 @@ template <typename T, int L, int V> struct LaunchV {
     a.ntile = int((a.ninner + NC - 1) / NC);
     const long long gx = a.ntile * nouter;
     if (gx <= 0 || gx > 0x7fffffffLL || nmem > 65535) return cudaErrorInvalidValue;
-    return launch_pass(k, dim3(unsigned(gx), ncomp, nmem), NC * TPL, smem, st, a.pdl, a);
+    return launch_pass(k, dim3(unsigned(gx), ncomp, nmem), NC * TPL, smem, st, a);
   }
 
   // The padding and truncating passes of the 3/2 rule (n == 2L/3) take the
@@ -234,7 +236,7 @@ template <typename T, int L, int V> struct LaunchV {
     if (attr != cudaSuccess) return attr;
     a.ntile = int((a.ninner + NCM - 1) / NCM);
     if (nmem > 65535) return cudaErrorInvalidValue;
-    return launch_pass(k, dim3(unsigned(a.ntile), nmem), NB * NCM * TPL, smem, st, a.pdl, a);
+    return launch_pass(k, dim3(unsigned(a.ntile), nmem), NB * NCM * TPL, smem, st, a);
   }
 
   template <int NCM> static cudaError_t epi_std(const EpiArgs& a, unsigned nmem, cudaStream_t st) {
@@ -305,7 +307,7 @@ template <typename T, int L> struct LaunchZ {
     const long long chunks = (a.nlines + 2 * NLP - 1) / (2 * NLP);
     if (chunks == 0 || a.nmem == 0) return cudaSuccess;
     if (chunks > 0x7fffffffLL || a.nmem > 65535) return cudaErrorInvalidValue;
-    return launch_pass(k, dim3(unsigned(chunks), unsigned(a.nmem)), Z::NT, size_t(smem), st, 1, a);
+    return launch_pass(k, dim3(unsigned(chunks), unsigned(a.nmem)), Z::NT, size_t(smem), st, a);
   }
   template <int DIM, int NLP> static cudaError_t run(const ZArgs& a, cudaStream_t st) {
     if constexpr (L % 3 == 0) {
@@ -339,7 +341,7 @@ template <typename T, int L> struct LaunchZ {
     const long long chunks = (a.nlines + 2 * NLP - 1) / (2 * NLP);
     if (chunks == 0 || a.nmem == 0) return cudaSuccess;
     if (chunks > 0x7fffffffLL || a.nmem > 65535) return cudaErrorInvalidValue;
-    return launch_pass(k, dim3(unsigned(chunks), unsigned(a.nmem)), Z::NT, size_t(smem), st, 1, a, pstride);
+    return launch_pass(k, dim3(unsigned(chunks), unsigned(a.nmem)), Z::NT, size_t(smem), st, a, pstride);
   }
   static cudaError_t product(int dim, const ZArgs& a, cudaStream_t st) {
     if (dim == 2) return run<2>(a, st);
@@ -362,7 +364,7 @@ template <typename T, int L> struct LaunchLine {
     a.ntile = int((a.ninner + Tile::NC - 1) / Tile::NC);
     const long long gx = a.ntile * nouter;
     if (gx <= 0 || gx > 0x7fffffffLL || nmem > 65535) return cudaErrorInvalidValue;
-    return launch_pass(k, dim3(unsigned(gx), 1, nmem), Tile::NT, smem, st, a.pdl, a);
+    return launch_pass(k, dim3(unsigned(gx), 1, nmem), Tile::NT, smem, st, a);
   }
   template <typename Tile, int MODE>
   static cudaError_t col_std(const ColArgs& a, long long nouter, unsigned nmem, cudaStream_t st) {
@@ -397,7 +399,7 @@ template <typename T, int L> struct LaunchLine {
     if (attr != cudaSuccess) return attr;
     a.ntile = int((a.ninner + Tile::NCM - 1) / Tile::NCM);
     if (nmem > 65535) return cudaErrorInvalidValue;
-    return launch_pass(k, dim3(unsigned(a.ntile), nmem), Tile::NT, smem, st, a.pdl, a);
+    return launch_pass(k, dim3(unsigned(a.ntile), nmem), Tile::NT, smem, st, a);
   }
   template <typename Tile> static cudaError_t epi_std(const EpiArgs& a, unsigned nmem, cudaStream_t st) {
     if constexpr (L % 3 == 0) {

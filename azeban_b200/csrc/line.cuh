@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(NT, MINB) k_epilogue2d(EpiArgs a) {
   C* tws = reinterpret_cast<C*>(az_smem);
   C* twm = tws + (P::RB - 1) * P::S;
   C* sm = tws + Sh::TW;
-  pdl_enter();
+  if (a.pdl) pdl_enter();
   const int member = blockIdx.y;
   if (a.ctrl != nullptr && a.ctrl[member].skip) return;
   __shared__ double step_dt;

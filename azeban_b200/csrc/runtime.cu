@@ -363,6 +363,7 @@ static cudaError_t product_pass(az_euler e, int dim, ZArgs& z, cudaStream_t st) 
   z.norm = e->norm;
   z.ctrl = e->ctrl;
   z.wait_polls = g_wait_polls;
+  z.pdl = 1;
   return e->ks->product(dim, z, st);
 }
 

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(ZFShape<T, L, NLP, VF, VI>::NT, ZFShape<T, L, 
   C* w = reinterpret_cast<C*>(az_smem + Z::OFF_W);
   const int member = blockIdx.y;
   Ctrl* ctrl = a.ctrl + member;
-  pdl_enter();
+  if (a.pdl) pdl_enter();
   if (ctrl->skip) return;
   const int tid = threadIdx.x;
   const int nh = STD ? L / 3 + 1 : a.nh;

@@ -117,6 +117,7 @@ struct ZArgs {
   double norm;       // 1 / (N^{d/2} M^{d/2})
   Ctrl* ctrl;
   int wait_polls;    // limit of the wait for the chunk's bulk copy (kWaitPolls)
+  int pdl;           // programmatic dependent launch
 };
 
 // Product c of the velocities u (kProducts): in 2-D 11, 12, 22; in 3-D the
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(ZLineShape<T, L, NLP, DIM>::NT, ZLineShape<T, 
   C* w = reinterpret_cast<C*>(az_smem + Z::OFF_W);
   const int member = blockIdx.y;
   Ctrl* ctrl = a.ctrl + member;
-  pdl_enter();
+  if (a.pdl) pdl_enter();
   if (ctrl->skip) return;
   const int tid = threadIdx.x;
   const int nh = STD ? L / 3 + 1 : a.nh;
