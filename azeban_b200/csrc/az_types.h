@@ -35,24 +35,14 @@ struct Visc {
   long long N;
 };
 
-// Products of velocities that a right-hand side on the padded length L
-// transforms: all three of u (x) u in 2-D; in 3-D u (x) u without its trace (5;
-// product() in zline.cuh says why that is enough), all six at L = 384.
-// In 2-D the trace stays: in a shear flow u_x(y) the rounding of u_x^2 is the same
-// on every line x = const, so it has no part in kx != 0; u_x^2 - u_y^2 is rounded
-// differently on each (right-hand side of a 128^2 FP32 double shear layer 2.9e-5
-// off FP64 instead of 5e-6).
-// In 3-D the same happens only to an exact shear flow whose z velocity varies
-// across it (32^3, single precision on the CPU: u_x(z), u_z(x) 7.3e-6 instead of
-// 1.1e-6); flows with u_z = 0, random fields and vortices are as accurate with five
-// products as with six (64^3 to 512^3: within 2 % of each other against FP64).
-// There the five-product form (1.23x faster on other lengths, 17.4 -> 14.7 ms a
-// step on four 256^3 FP32 members) is as far from FP64 as the six-product form
-// (relative L2 error of a 256^3 Taylor-Green step, its leading modes left out:
-// 2.5e-6 both in FP32, 7.1e-15 both in FP64), but the two differ at single modes by up
-// to 1.2e-3 (FP32) and 2.6e-12 (FP64) of the root mean square, more than results
-// of these workloads may change from one version to the next.
-template <int DIM, int L> inline constexpr int kProducts = DIM == 2 ? 3 : L == 384 ? 6 : 5;
+// Products of velocities that a right-hand side transforms: the entries of u (x) u on and
+// below its diagonal.  (A multiple of the identity adds only a gradient, which the
+// projection removes, so five would do in 3-D, 11 - 33, 21, 22 - 33, 31, 32, and 1.1 times
+// as fast.  But the rounding of a large u_z^2 then enters equations that 33 itself, which
+// meets nothing but k_z, has no part in: two crossing shear layers with u_x / u_z = 0.01
+// were off FP64 by 2.4e-5 instead of 1e-6 in FP32, a jet along z with a hundredth of its
+// velocity across it by 2e-5 instead of 3e-7, the same flows along x not at all.)
+constexpr int products(int dim) { return dim * (dim + 1) / 2; }
 
 enum Mode : int { MODE_DUDT = 0, MODE_RK1 = 1, MODE_RK2 = 2, MODE_RK3 = 3 };
 

@@ -6,19 +6,19 @@
 // passes, each one HBM read and one HBM write of the live array.  The
 // intermediates keep the component index innermost, so a tile of consecutive
 // columns is one contiguous run per row in every pass:
-//   1 k_cols<PAD,  inverse>  along x: u_hat [3][N][N][Nh] -> A1 [M][N][Nh][3]
-//                            (copy_to_padded along x fused into the loads)
-//   2 k_cols<PAD,  inverse>  along y: A1 -> A2 [M][M][Nh][3]
-//   3 k_zline                along z: c2r, max|u|, B = u (x) u, r2c, keep
-//                            k < Nh: A2 -> B1 [M][M][Nh][5] (6 products at M = 384, by
-//                            k_zfused)
-//   4 k_cols<TRUNC, forward> along y, keep the N retained rows: B1 -> B2 [M][N][Nh][5]
-//   5 k_fwd_epilogue         along x, keep retained rows, then computeDudt
-//                            (Leray projection of i k.B, spectral viscosity)
-//                            and the SSP-RK3 stage combination: B2 + u -> out
+//   1 k_columns<PAD>    inverse along x: u_hat [3][N][N][Nh] -> A1 [M][N][Nh][3]
+//                       (copy_to_padded along x fused into the loads)
+//   2 k_columns<PAD>    inverse along y: A1 -> A2 [M][M][Nh][3]
+//   3 k_zline           along z: c2r, max|u|, B = u (x) u, r2c, keep k < Nh:
+//                       A2 -> B1 [M][M][Nh][6]
+//   4 k_columns<TRUNC>  forward along y, keep the N retained rows: B1 -> B2 [M][N][Nh][6]
+//   5 k_fwd_epilogue    forward along x, keep retained rows, then computeDudt
+//                       (Leray projection of i k.B, spectral viscosity)
+//                       and the SSP-RK3 stage combination: B2 + u -> out
 // 2-D uses passes 1 (along x), 3 (along y) and a last pass k_epilogue2d, with A1
-// [M][Nh][2] and B1 [M][Nh][3].  Passes 1 and 2 are k_pad_inverse (line.cuh), or
-// k_cols in 3-D at M = 384 (kProducts); pass 3 is k_zline (zline.cuh).
+// [M][Nh][2] and B1 [M][Nh][3].  k_columns and k_epilogue2d are in line.cuh, k_zline
+// in zline.cuh; 3-D solves with M = 384 have k_cols and k_zfused (zfused.cuh) in their
+// place (kRegisterColumns).
 #pragma once
 
 #include "az_types.h"
@@ -237,7 +237,7 @@ template <typename T> __device__ __forceinline__ double epilogue_dt(const EpiArg
   return dt;
 }
 
-// Forward transform along x of the NB product components (kProducts), kept at the N
+// Forward transform along x of the six product components, kept at the N
 // retained rows, then per mode: L = (I - k k^T/|k|^2)(i k.B_hat),
 // dudt = |k| = 0 ? 0 : -L + nu(|k|) u_hat (incompressible_euler.hpp:230-347,
 // incompressible_euler_functions.hpp:47-112), then the stage combination:
@@ -249,19 +249,19 @@ template <typename T> __device__ __forceinline__ double epilogue_dt(const EpiArg
 // FP32 std plans of up to 384 threads: two resident CTAs per SM.
 template <typename T, int L, int NCM, int V> struct EpiMinBlocks {
   static constexpr int value =
-      (sizeof(T) == 4 && V == 0 && kProducts<3, L> * NCM * Plan<L, V>::TPL <= 384) ? 2 : 1;
+      (sizeof(T) == 4 && V == 0 && products(3) * NCM * Plan<L, V>::TPL <= 384) ? 2 : 1;
 };
 
 // STD: N == 2L/3 (the 3/2 rule), known at compile time, so the retained-row
 // map and the per-mode row loops fold.
 template <typename T, int L, int NCM, int V, bool STD>
-__global__ void __launch_bounds__(kProducts<3, L> * NCM * Plan<L, V>::TPL,
+__global__ void __launch_bounds__(products(3) * NCM * Plan<L, V>::TPL,
                                   EpiMinBlocks<T, L, NCM, V>::value)
     k_fwd_epilogue(EpiArgs a) {
   using C = cvec<T>;
   using P = Plan<L, V>;
   constexpr int DIM = 3;
-  constexpr int NB = kProducts<3, L>;
+  constexpr int NB = products(DIM);
   constexpr int NC = NB * NCM;
   constexpr int SROW = NC;
   constexpr int TPL = P::TPL;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kProducts<3, L> * NCM * Plan<L, V>::TPL,
     const int i_ = i >= N / 2 + 1 ? i - N : i;
     const T k1 = twopi * T(i_);
     C Bv[NB];
-    if constexpr (sizeof(C) == 8 && NB % 2 == 0) {
+    if constexpr (sizeof(C) == 8) {
       // 16-byte reads: with rows of NB * NCM elements a quarter-warp's reads
       // fall on distinct bank groups
       const float4* b4 = reinterpret_cast<const float4*>(sm + i * SROW + pl * NB);
@@ -375,14 +375,13 @@ __global__ void __launch_bounds__(kProducts<3, L> * NCM * Plan<L, V>::TPL,
     C Lh[DIM];
     T absk2;
     absk2 = k1 * k1 + k2 * k2 + k3 * k3;
-    // B order: 0 B11 (- B33), 1 B21, 2 B22 (- B33), 3 B31, 4 B32, 5 B33 of six products
+    // B order: 0 B11, 1 B21, 2 B22, 3 B31, 4 B32, 5 B33
     const C b1 = cmk<C>(-k1 * Bv[0].y - k2 * Bv[1].y - k3 * Bv[3].y,
                         k1 * Bv[0].x + k2 * Bv[1].x + k3 * Bv[3].x);
     const C b2 = cmk<C>(-k1 * Bv[1].y - k2 * Bv[2].y - k3 * Bv[4].y,
                         k1 * Bv[1].x + k2 * Bv[2].x + k3 * Bv[4].x);
-    const C b3 = NB == 6 ? cmk<C>(-k1 * Bv[3].y - k2 * Bv[4].y - k3 * Bv[NB - 1].y,
-                                  k1 * Bv[3].x + k2 * Bv[4].x + k3 * Bv[NB - 1].x)
-                         : cmk<C>(-k1 * Bv[3].y - k2 * Bv[4].y, k1 * Bv[3].x + k2 * Bv[4].x);
+    const C b3 = cmk<C>(-k1 * Bv[3].y - k2 * Bv[4].y - k3 * Bv[5].y,
+                        k1 * Bv[3].x + k2 * Bv[4].x + k3 * Bv[5].x);
     const T inv = T(1) / absk2;
     const C sk = cmk<C>((k1 * b1.x + k2 * b2.x + k3 * b3.x) * inv, (k1 * b1.y + k2 * b2.y + k3 * b3.y) * inv);
     Lh[0] = cmk<C>(b1.x - k1 * sk.x, b1.y - k1 * sk.y);

@@ -13,9 +13,9 @@
 
 namespace azb {
 
-// KernelSet::cols takes the plain kinds and, for the six-product form only
-// (kProducts), COLK_PAD_INV and COLK_TRUNC_FWD; else those are KernelSet::columns',
-// with COLK_PAD_STATE, the padding pass that reads the state.
+// KernelSet::cols takes the plain kinds and, where reg3 is set, COLK_PAD_INV and
+// COLK_TRUNC_FWD; else those are KernelSet::columns', with COLK_PAD_STATE, the padding
+// pass that reads the state.
 enum ColKind : int { COLK_PAD_INV = 0, COLK_PLAIN_INV = 1, COLK_TRUNC_FWD = 2, COLK_PLAIN_FWD = 3, COLK_PAD_STATE = 4 };
 
 // v: plan variant (0 std, 1 wide; see Plan<L, V>).  The launchers pick the tile
@@ -23,7 +23,7 @@ enum ColKind : int { COLK_PAD_INV = 0, COLK_PLAIN_INV = 1, COLK_TRUNC_FWD = 2, C
 struct KernelSet {
   int L;
   int precision;  // 0 FP64, 1 FP32
-  int nb3;        // products of a 3-D right-hand side
+  bool reg3;      // 3-D solves take cols and the product pass k_zfused (kRegisterColumns)
   cudaError_t (*cols)(int v, int kind, const ColArgs&, long long nouter, unsigned ncomp, unsigned nmem, cudaStream_t);
   cudaError_t (*product)(int dim, const ZArgs&, cudaStream_t);
   // kinds COLK_PAD_INV, COLK_PAD_STATE and COLK_TRUNC_FWD
@@ -34,6 +34,17 @@ struct KernelSet {
   cudaError_t (*c2r)(const RealRowArgs&, cudaStream_t);
   cudaError_t (*r2c)(int v, const RealRowArgs&, cudaStream_t);
 };
+
+// Lengths whose 3-D passes keep a column in the registers of a few threads (k_cols,
+// k_zfused) instead of k_columns and k_zline.  At 384 the latter are faster under the
+// 3/2 rule (a step of four 256^3 FP32 members 16400 us against 17500, of one in FP64 8280
+// against 9370; with N = 214 4810 against 4120 in FP32, 6780 against 8080 in FP64) and as
+// far from FP64, 3.1e-6 and 8e-15 in the 2-norm of a Taylor-Green step without its leading
+// modes.  But they add in another order, and single modes beside the leading ones move by
+// up to 1.2e-3 (FP32) and 6e-12 (FP64) of the root mean square of the others (either form
+// is half as far from FP64 there), which the tolerance of the 256^3 vortex solves in
+// perf/cases.py does not allow.
+template <int L> inline constexpr bool kRegisterColumns = L == 384;
 
 constexpr int kpow2floor(int x) {
   int p = 1;
@@ -53,12 +64,13 @@ template <typename T, int L, int V> struct Tiles {
 };
 
 // Line pairs per CTA of the product pass.  Wide: about 96 threads (one
-// middle-stage butterfly each), 128 for the plans with RM = 12 and 192 where a
-// pair has 96 in FP32 (measured best of 1 to 12 pairs).  Narrow: one warp, taken
-// when the wide chunks would not give every SM its CTAs.
+// middle-stage butterfly each), 128 for the plans with RM = 12 and, in 2-D, 192 where
+// a pair has 96 in FP32 (measured best of 1 to 12 pairs; in 3-D L = 768 takes 4148 us
+// with one pair and 4557 with two).  Narrow: one warp, taken when the wide chunks
+// would not give every SM its CTAs.
 template <typename T, int L, int DIM> struct ZLineTile {
   static constexpr int S = L / ZPlan<T, L, DIM>::RM;
-  static constexpr int WIDE = S >= 96 ? (sizeof(T) == 4 && S == 96 ? 2 : 1)
+  static constexpr int WIDE = S >= 96 ? (DIM == 2 && sizeof(T) == 4 && S == 96 ? 2 : 1)
                               : ZPlan<T, L, DIM>::RM == 12 ? (128 / S) : (96 / S);
   static constexpr int NARROW = S >= 32 ? 1 : 32 / S;
 };
@@ -217,11 +229,11 @@ template <typename T, int L, int V> struct LaunchV {
     constexpr int NC = TS::NC;
     switch (kind) {
       case COLK_PAD_INV:
-        if constexpr (kProducts<3, L> == 6) return col_std<+1, COL_PAD, NC>(a, nouter, ncomp, nmem, st);
+        if constexpr (kRegisterColumns<L>) return col_std<+1, COL_PAD, NC>(a, nouter, ncomp, nmem, st);
         else return cudaErrorInvalidValue;
       case COLK_PLAIN_INV: return col_std<+1, COL_PLAIN, NC>(a, nouter, ncomp, nmem, st);
       case COLK_TRUNC_FWD:
-        if constexpr (kProducts<3, L> == 6) return col_std<-1, COL_TRUNC, NC>(a, nouter, ncomp, nmem, st);
+        if constexpr (kRegisterColumns<L>) return col_std<-1, COL_TRUNC, NC>(a, nouter, ncomp, nmem, st);
         else return cudaErrorInvalidValue;
       case COLK_PLAIN_FWD: return col_std<-1, COL_PLAIN, NC>(a, nouter, ncomp, nmem, st);
       default: return cudaErrorInvalidValue;
@@ -229,7 +241,7 @@ template <typename T, int L, int V> struct LaunchV {
   }
 
   template <int NCM, bool STD> static cudaError_t epi_run(EpiArgs a, unsigned nmem, cudaStream_t st) {
-    constexpr int NB = kProducts<3, L>;
+    constexpr int NB = products(3);
     const size_t smem = size_t(L + L * NB * NCM) * sizeof(C);
     auto k = k_fwd_epilogue<T, L, NCM, V, STD>;
     static const cudaError_t attr = set_smem(k, smem);
@@ -322,9 +334,9 @@ template <typename T, int L> struct LaunchZ {
     }
     return run<DIM, Z::WIDE>(a, st);
   }
-  // Six products: the forward transforms on the wide plan, the inverse on the
-  // std plan, four line pairs per CTA in FP32 and two in FP64 (some 80 KB).
-  template <bool STD> static cudaError_t run_six(const ZArgs& a, cudaStream_t st) {
+  // k_zfused: the forward transforms on the wide plan, the inverse on the std
+  // plan, four line pairs per CTA in FP32 and two in FP64 (some 80 KB).
+  template <bool STD> static cudaError_t run_fused(const ZArgs& a, cudaStream_t st) {
     constexpr int NLP = sizeof(T) == 4 ? 4 : 2;
     using Z = ZFShape<T, L, NLP, 1, 0>;
     if (a.in_line < a.nh * 3 || a.out_line < a.nh * Z::NB) return cudaErrorInvalidValue;
@@ -346,8 +358,8 @@ template <typename T, int L> struct LaunchZ {
   static cudaError_t product(int dim, const ZArgs& a, cudaStream_t st) {
     if (dim == 2) return run<2>(a, st);
     if (dim != 3) return cudaErrorInvalidValue;
-    if constexpr (kProducts<3, L> == 6)
-      return a.nh == L / 3 + 1 ? run_six<true>(a, st) : run_six<false>(a, st);
+    if constexpr (kRegisterColumns<L>)
+      return a.nh == L / 3 + 1 ? run_fused<true>(a, st) : run_fused<false>(a, st);
     else
       return run<3>(a, st);
   }
@@ -434,7 +446,7 @@ template <typename T, int L> struct Launch {
   static const KernelSet* get() {
     static const KernelSet ks = {L,
                                  sizeof(T) == 8 ? 0 : 1,
-                                 kProducts<3, L>,
+                                 kRegisterColumns<L>,
                                  &cols,
                                  &LaunchZ<T, L>::product,
                                  &LaunchLine<T, L>::columns,

@@ -236,9 +236,12 @@ template <typename T, typename P, int NCM> struct Epi2Shape {
 };
 
 // Last pass of a 2-D right-hand side: forward along x of B11 - B22 and B12 (a
-// transform fewer; the difference is taken here, on values already transformed
-// along y, where the terms of a shear flow share no wavenumber that matters, see
-// kProducts), kept at the N retained rows, then per mode dudt = |k| = 0 ? 0 : -L +
+// transform fewer; the projection meets them as this difference alone, with one factor,
+// so rounding has the same weights as with both.  It is taken here, on values already
+// transformed along y: in a shear flow u_x(y) the rounding of u_x^2 is the same on every
+// line x = const and has no part in kx != 0, but that of u_x^2 - u_y^2 is another on each,
+// and a product pass that took it put a 128^2 FP32 double shear layer 2.9e-5 off FP64
+// instead of 5e-6), kept at the N retained rows, then per mode dudt = |k| = 0 ? 0 : -L +
 // nu(|k|) u_hat with L the projected divergence (incompressible_euler.hpp:230-347,
 // incompressible_euler_functions.hpp:47-112), which in 2-D is
 //   L_x = i ky q / k^2, L_y = -i kx q / k^2,

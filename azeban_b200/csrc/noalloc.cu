@@ -80,7 +80,7 @@ az_status az_euler_dudt_noalloc(int dim, long long N_phys, long long N_phys_pad,
   e.N = N_phys;
   e.M = N_phys_pad;
   e.Nh = e.N / 2 + 1;
-  e.nb = dim == 3 ? ks->nb3 : 3;
+  e.nb = products(dim);
   e.visc.type = visc->type;
   e.visc.eps = visc->eps;
   e.visc.s = visc->s;

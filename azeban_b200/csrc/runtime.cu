@@ -276,7 +276,7 @@ az_status az_euler_create(const az_euler_desc* d, az_euler* out) {
   e->N = d->N_phys;
   e->M = d->N_phys_pad;
   e->Nh = e->N / 2 + 1;
-  e->nb = e->dim == 3 ? ks->nb3 : 3;
+  e->nb = products(e->dim);
   e->visc.type = d->visc.type;
   e->visc.eps = d->visc.eps;
   e->visc.s = d->visc.s;
@@ -396,7 +396,6 @@ static az_status rhs(az_euler e, const void* u, bool u_inner, const void* u0, bo
   if (e->dim == 3) {
     // pass 1: inverse along x with padding, state [3][N][N][Nh] -> A1 [M][N][r3]
     // (column p: group y = p / r3, entry q = 3 z + component, q < 3 Nh)
-    const bool six = e->nb == 6;  // k_cols (kProducts)
     ColArgs a1{};
     a1.in = u;
     a1.out = e->buf[0];
@@ -423,7 +422,7 @@ static az_status rhs(az_euler e, const void* u, bool u_inner, const void* u0, bo
     a1.pdl = begin == BEGIN_NONE;
     {
       ProfScope ps(P_INV_X, double(B) * 3 * (N * N * Nh + M * N * Nh) * e->csize, st, e->prof);
-      ce = six ? ks->cols(e->v_cols, COLK_PAD_INV, a1, 1, 1, B, st) : ks->columns(COLK_PAD_STATE, a1, 1, B, st);
+      ce = ks->reg3 ? ks->cols(e->v_cols, COLK_PAD_INV, a1, 1, 1, B, st) : ks->columns(COLK_PAD_STATE, a1, 1, B, st);
     }
     if (ce != cudaSuccess) return cuda_fail(ce, "rhs pass 1");
     // pass 2: inverse along y with padding, A1 -> A2 [M][M][r3]
@@ -444,10 +443,10 @@ static az_status rhs(az_euler e, const void* u, bool u_inner, const void* u0, bo
     a2.pdl = 1;
     {
       ProfScope ps(P_INV_Y, double(B) * 3 * (M * N * Nh + M * M * Nh) * e->csize, st, e->prof);
-      ce = six ? ks->cols(e->v_cols, COLK_PAD_INV, a2, M, 1, B, st) : ks->columns(COLK_PAD_INV, a2, M, B, st);
+      ce = ks->reg3 ? ks->cols(e->v_cols, COLK_PAD_INV, a2, M, 1, B, st) : ks->columns(COLK_PAD_INV, a2, M, B, st);
     }
     if (ce != cudaSuccess) return cuda_fail(ce, "rhs pass 2");
-    // pass 3: z lines, product, CFL max: A2 -> B1 [M][M][r5]
+    // pass 3: z lines, product, CFL max: A2 -> B1 [M][M][r6]
     ZArgs z{};
     z.in = e->buf[1];
     z.out = e->buf[2];
@@ -503,7 +502,7 @@ static az_status rhs(az_euler e, const void* u, bool u_inner, const void* u0, bo
   const char* bsrc;
   long long b_row, b_mem, ninner;
   if (e->dim == 3) {
-    // pass 4: forward along y, keep retained rows: B1 -> B2 [M][N][r5]
+    // pass 4: forward along y, keep retained rows: B1 -> B2 [M][N][r6]
     ColArgs a4{};
     a4.in = e->buf[2];
     a4.out = e->buf[0];
@@ -521,7 +520,7 @@ static az_status rhs(az_euler e, const void* u, bool u_inner, const void* u0, bo
     a4.pdl = 1;
     {
       ProfScope ps(P_FWD_Y, double(B) * e->nb * (M * M * Nh + M * N * Nh) * e->csize, st, e->prof);
-      ce = e->nb == 6 ? ks->cols(e->v_cols, COLK_TRUNC_FWD, a4, M, 1, B, st) : ks->columns(COLK_TRUNC_FWD, a4, M, B, st);
+      ce = ks->reg3 ? ks->cols(e->v_cols, COLK_TRUNC_FWD, a4, M, 1, B, st) : ks->columns(COLK_TRUNC_FWD, a4, M, B, st);
     }
     if (ce != cudaSuccess) return cuda_fail(ce, "rhs pass 4");
     bsrc = e->buf[0];

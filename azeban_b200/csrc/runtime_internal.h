@@ -15,7 +15,7 @@ struct az_euler_s {
   // touched.
   int nlaunch = 0;
   long long N, M, Nh;
-  int nb;  // products of a right-hand side (kProducts)
+  int nb;  // products of a right-hand side
   azb::Visc visc;
   double eps_visc;  // Equation::visc()
   const azb::KernelSet* ks;

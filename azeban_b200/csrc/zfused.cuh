@@ -1,4 +1,4 @@
-// Contiguous-axis pass of the six-product right-hand sides (kProducts): c2r of
+// Contiguous-axis pass of 3-D right-hand sides at the lengths of kRegisterColumns: c2r of
 // the velocity lines, the CFL maximum, B = u (x) u in the reference's component
 // order, r2c of the products, bins [0, nh) kept, with the products fused into
 // the forward transform's loads:

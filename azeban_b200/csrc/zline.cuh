@@ -28,10 +28,9 @@
 // What bounds it: issue and the latency of 12 to 18 resident warps per SM; it
 // executes some 250 instructions per row of a line pair, of which 200 are FP32
 // arithmetic.  Against the earlier form, whose velocities and products went
-// through shared memory (67 shared accesses per row of a pair instead of 23) and
-// which transformed six products (us, before -> after): 512^3 FP32 5700 -> 3650,
-// 64^3 x15 FP32 138 -> 89, 128^3 FP64 157 -> 114; 2-D (three products in both)
-// 128^2 x256 FP32 63 -> 45, 512^2 x64 252 -> 209, 1024^2 FP64 98 -> 40.
+// through shared memory (67 shared accesses per row of a pair instead of 25; us,
+// before -> after): 512^3 FP32 5700 -> 4160, 64^3 x15 FP32 138 -> 91, 128^3 FP64 157 -> 122;
+// 2-D 128^2 x256 FP32 63 -> 45, 512^2 x64 252 -> 209, 1024^2 FP64 98 -> 40.
 //
 // Reference: the inverse transform, max_norm and computeB of
 // IncompressibleEuler::dudt (include/azeban/equations/incompressible_euler.hpp
@@ -51,12 +50,12 @@ namespace azb {
 // (the separation pairs butterflies j and L/R1 - j).  A larger RM makes the
 // outer stages fewer or smaller, a smaller one leaves registers for more
 // resident warps, which the pass is short of.  Measured on 2.4e8 padded points
-// (FP32, 3-D; us): 384 as 32.12 1558, 24.16 1852, 8.6.8 1808, 48.8 2348; 768 as
-// 12.8.8 3631, 8.6.16 4860, 16.4.12 4052; 192 as 16.12 1479, 12.16 1811.  In FP64
-// (6e7 points): 384 as 12.8.4 868, 8.8.6 890, 8.6.8 992; 192 as 12.4.4 836, 24.8
-// 882.  In 2-D a thread holds two components, so RM is larger (figures with two
-// products): FP32 384 as 24.16 810, 32.12 995; 192 as 12.16 815, 16.12 885; FP64
-// 384 as 8.6.8 474, 12.8.4 525.
+// (FP32, 3-D; us): 192 as 16.12 1603, 24.8 1751, 12.2.8 2146, 8.3.8 2133; 768 as 12.8.8
+// 4148; with one product fewer 384 as 32.12 1558, 24.16 1852, 8.6.8 1808, 48.8 2348; 768
+// as 12.8.8 3631, 8.6.16 4860, 16.4.12 4052.  In FP64 (6e7 points; one product fewer):
+// 384 as 12.8.4 868, 8.8.6 890, 8.6.8 992; 192 as 12.4.4 836, 24.8 882.  In 2-D a thread
+// holds two components, so RM is larger (one product fewer): FP32 384 as 24.16 810,
+// 32.12 995; 192 as 12.16 815, 16.12 885; FP64 384 as 8.6.8 474, 12.8.4 525.
 template <typename T, int L, int DIM> struct ZPlan;
 #define AZB_ZPLAN(Tv, Lv, A3, B3, M3, A2, B2, M2)              \
   template <> struct ZPlan<Tv, Lv, 3> {                        \
@@ -120,22 +119,11 @@ struct ZArgs {
   int pdl;           // programmatic dependent launch
 };
 
-// Product c of the velocities u (kProducts): in 2-D 11, 12, 22; in 3-D the
-// components of u (x) u with its last diagonal entry taken off the diagonal,
-// 11 - 33, 21, 22 - 33, 31, 32.  A multiple of the identity adds i s k to the divergence
-// i k.B, which the projection removes exactly, so the right-hand side is the
-// same with one transform fewer (products of the reference:
-// include/azeban/equations/incompressible_euler_functions.hpp:26-45).
+// Product c of the velocities u: 11, 12, 22 in 2-D; 11, 21, 22, 31, 32, 33 in 3-D
+// (include/azeban/equations/incompressible_euler_functions.hpp:26-45).
 template <int DIM, int c, typename T> __device__ __forceinline__ T product(const T (&u)[DIM]) {
-  if constexpr (DIM == 2) {
-    return c == 0 ? u[0] * u[0] : c == 1 ? u[0] * u[1] : u[1] * u[1];
-  } else {
-    if constexpr (c == 0) return (u[0] - u[2]) * (u[0] + u[2]);
-    if constexpr (c == 1) return u[1] * u[0];
-    if constexpr (c == 2) return (u[1] - u[2]) * (u[1] + u[2]);
-    if constexpr (c == 3) return u[2] * u[0];
-    return u[2] * u[1];
-  }
+  constexpr int i = c == 0 ? 0 : c < 3 ? 1 : 2;
+  return u[i] * u[c - i * (i + 1) / 2];
 }
 
 // Shared memory of one CTA: the mbarrier, the middle stage's twiddles
@@ -145,7 +133,7 @@ template <int DIM, int c, typename T> __device__ __forceinline__ T product(const
 template <typename T, int L, int NLP, int DIM> struct ZLineShape {
   using P = ZPlan<T, L, DIM>;
   static constexpr int CB = int(sizeof(cvec<T>));
-  static constexpr int NB = DIM == 3 ? 5 : 3;
+  static constexpr int NB = products(DIM);
   static constexpr int S = L / P::RM;       // rows (middle-stage butterflies) of a pair
   static constexpr int SV = (P::RM * DIM) | 1;
   static constexpr int SP = (P::RM * NB) | 1;
@@ -155,10 +143,12 @@ template <typename T, int L, int NLP, int DIM> struct ZLineShape {
   // radices, which need them, 15 (128 registers) or, with whole CTAs of 192
   // threads, 18 for the others.
   static constexpr int WARPS = P::RM * CB > 64 ? 12 : NT == 192 && CB == 8 ? 18 : 15;
-  static constexpr int MINB = NT < WARPS * 32 ? WARPS * 32 / NT : 1;
   static constexpr int NTW = (P::RM - 1) * S + (P::R2 - 1) * P::R1;
   static constexpr int OFF_TW = 16;
   static constexpr int OFF_W = (OFF_TW + NTW * CB + 15) / 16 * 16;
+  // resident CTAs by registers and by the product rows' shared memory
+  static constexpr int FIT = 228 * 1024 / (OFF_W + NLP * PP * CB + 1024);
+  static constexpr int MINB = FIT < 2 || NT >= WARPS * 32 ? 1 : FIT < WARPS * 32 / NT ? FIT : WARPS * 32 / NT;
   static constexpr int V_END = (NLP * VP * CB + 15) / 16 * 16;  // bytes
   static __host__ __device__ int in_off(int in_line) {  // bytes from OFF_W to the input
     const int at_end = NLP * (PP * CB - 2 * in_line * CB) / 16 * 16;
@@ -359,7 +349,7 @@ __global__ void __launch_bounds__(ZLineShape<T, L, NLP, DIM>::NT, ZLineShape<T, 
         }
       }
       C* dst = w + p * Z::PP + s * SP;
-auto one = [&](auto cc) {
+      auto one = [&](auto cc) {
         constexpr int c = decltype(cc)::value;
         C t[RM];
 #pragma unroll
@@ -382,6 +372,7 @@ auto one = [&](auto cc) {
       if constexpr (DIM == 3) {
         one(std::integral_constant<int, 3>{});
         one(std::integral_constant<int, 4>{});
+        one(std::integral_constant<int, 5>{});
       }
     }
   }
