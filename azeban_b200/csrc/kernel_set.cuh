@@ -64,15 +64,16 @@ template <typename T, int L, int V> struct Tiles {
 };
 
 // Line pairs per CTA of the product pass.  Wide: about 96 threads (one
-// middle-stage butterfly each), 128 for the plans with RM = 12 and, in 2-D, 192 where
-// a pair has 96 in FP32 (measured best of 1 to 12 pairs; in 3-D L = 768 takes 4148 us
-// with one pair and 4557 with two).  Narrow: one warp, taken when the wide chunks
-// would not give every SM its CTAs.
+// middle-stage butterfly each), 128 for the plans with RM = 12 (measured best of 1 to
+// 12 pairs; L = 768 FP32 with one pair and with two: 3-D 4148 and 4557 us, 2-D 1220 and
+// 1267, off the 3/2 rule 1436 and 2037).  Narrow, taken when the wide chunks would not
+// give every SM its CTAs: one warp, or one pair where that is half a warp or more (two
+// of them take turns in the outer stages: a step of one 2-D N = 150
+// M = 256 FP32 solve 79 us with two pairs, 70 with one).
 template <typename T, int L, int DIM> struct ZLineTile {
   static constexpr int S = L / ZPlan<T, L, DIM>::RM;
-  static constexpr int WIDE = S >= 96 ? (DIM == 2 && sizeof(T) == 4 && S == 96 ? 2 : 1)
-                              : ZPlan<T, L, DIM>::RM == 12 ? (128 / S) : (96 / S);
-  static constexpr int NARROW = S >= 32 ? 1 : 32 / S;
+  static constexpr int WIDE = S >= 96 ? 1 : ZPlan<T, L, DIM>::RM == 12 ? 128 / S : 96 / S;
+  static constexpr int NARROW = S >= 16 ? 1 : 32 / S;
 };
 
 // Radix plans and tiles of the passes of line.cuh: columns (modes) of a tile,

@@ -50,12 +50,14 @@ namespace azb {
 // (the separation pairs butterflies j and L/R1 - j).  A larger RM makes the
 // outer stages fewer or smaller, a smaller one leaves registers for more
 // resident warps, which the pass is short of.  Measured on 2.4e8 padded points
-// (FP32, 3-D; us): 192 as 16.12 1603, 24.8 1751, 12.2.8 2146, 8.3.8 2133; 768 as 12.8.8
-// 4148; with one product fewer 384 as 32.12 1558, 24.16 1852, 8.6.8 1808, 48.8 2348; 768
-// as 12.8.8 3631, 8.6.16 4860, 16.4.12 4052.  In FP64 (6e7 points; one product fewer):
-// 384 as 12.8.4 868, 8.8.6 890, 8.6.8 992; 192 as 12.4.4 836, 24.8 882.  In 2-D a thread
-// holds two components, so RM is larger (one product fewer): FP32 384 as 24.16 810,
-// 32.12 995; 192 as 12.16 815, 16.12 885; FP64 384 as 8.6.8 474, 12.8.4 525.
+// (FP32, 3-D; us): 192 as 16.12 1603, 24.8 1751, 12.2.8 2146, 8.3.8 2133; 256 (N = 150)
+// as 8.4.8 2180, 4.8.8 2291, 16.16 2444, 16.2.8 2668, 32.8 3417 (2379 with registers for
+// 12 warps: a first stage of radix 32 off the 3/2 rule needs more than 128); 768 as
+// 12.8.8 4148; with one product fewer 384 as 32.12 1558, 24.16 1852, 8.6.8 1808, 48.8
+// 2348; 768 as 12.8.8 3631, 8.6.16 4860, 16.4.12 4052.  In FP64 (6e7 points; one product
+// fewer): 384 as 12.8.4 868, 8.8.6 890, 8.6.8 992; 192 as 12.4.4 836, 24.8 882.  In 2-D a
+// thread holds two components, so RM is larger (one product fewer): FP32 384 as 24.16
+// 810, 32.12 995; 192 as 12.16 815, 16.12 885; FP64 384 as 8.6.8 474, 12.8.4 525.
 template <typename T, int L, int DIM> struct ZPlan;
 #define AZB_ZPLAN(Tv, Lv, A3, B3, M3, A2, B2, M2)              \
   template <> struct ZPlan<Tv, Lv, 3> {                        \
@@ -78,7 +80,7 @@ AZB_ZPLAN(float, 64, 8, 1, 8, 8, 1, 8)
 AZB_ZPLAN(float, 96, 12, 1, 8, 12, 1, 8)
 AZB_ZPLAN(float, 128, 16, 1, 8, 8, 1, 16)
 AZB_ZPLAN(float, 192, 16, 1, 12, 12, 1, 16)
-AZB_ZPLAN(float, 256, 32, 1, 8, 16, 1, 16)
+AZB_ZPLAN(float, 256, 8, 4, 8, 16, 1, 16)
 AZB_ZPLAN(float, 384, 32, 1, 12, 24, 1, 16)
 AZB_ZPLAN(float, 512, 8, 8, 8, 32, 1, 16)
 AZB_ZPLAN(float, 768, 12, 8, 8, 12, 8, 8)
@@ -140,9 +142,9 @@ template <typename T, int L, int NLP, int DIM> struct ZLineShape {
   static constexpr int VP = S * SV, PP = S * SP;  // elements per pair
   static constexpr int NT = (NLP * S + 31) / 32 * 32;
   // Register cap: 12 resident warps per SM (168 registers) for the large middle
-  // radices, which need them, 15 (128 registers) or, with whole CTAs of 192
-  // threads, 18 for the others.
-  static constexpr int WARPS = P::RM * CB > 64 ? 12 : NT == 192 && CB == 8 ? 18 : 15;
+  // radices, which need them, 18 for the long FP32 lines of 2-D solves (L = 768 1220 us,
+  // with 15 warps 1294), 15 (128 registers) for the others.
+  static constexpr int WARPS = P::RM * CB > 64 ? 12 : DIM == 2 && CB == 8 && S >= 96 ? 18 : 15;
   static constexpr int NTW = (P::RM - 1) * S + (P::R2 - 1) * P::R1;
   static constexpr int OFF_TW = 16;
   static constexpr int OFF_W = (OFF_TW + NTW * CB + 15) / 16 * 16;
