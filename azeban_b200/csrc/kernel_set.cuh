@@ -146,8 +146,15 @@ template <typename T, int L> struct PadTileNarrow {
   static constexpr int NT = kclamp((NC * (P::O > P::S ? P::O : P::S) + 31) / 32 * 32, 32, 256);
   static constexpr int MINB = 1;
 };
+// The last pass of 2-D solves takes them for launches of at most one ordinary tile for
+// two SMs (10 FP32 solves with N = 214 and M = 384, 140 ordinary tiles: 113 us a step with
+// narrow ones, 89 without), and with radices that leave a thread of the last stage eight
+// rows instead of sixteen (one FP32 solve: N = 150, M = 256 70 -> 60; N = 298, M = 512 90 -> 72).
+template <typename T, int L> struct Epi2NarrowPlan { using P = typename Epi2Tile<T, L>::P; };
+template <> struct Epi2NarrowPlan<float, 256> { using P = LinePlan<float, 256, 32, 1, 8>; };
+template <> struct Epi2NarrowPlan<float, 512> { using P = LinePlan<float, 512, 8, 8, 8>; };
 template <typename T, int L> struct Epi2TileNarrow {
-  using P = typename Epi2Tile<T, L>::P;
+  using P = typename Epi2NarrowPlan<T, L>::P;
   static constexpr int NCM = 16 / int(sizeof(cvec<T>));
   static constexpr int NT = kclamp((NCM * (2 * P::O > P::S ? 2 * P::O : P::S) + 31) / 32 * 32, 32, 256);
   static constexpr int MINB = 1;
@@ -429,7 +436,7 @@ template <typename T, int L> struct LaunchLine {
     for (const StateLayout& l : {a.lu, a.lu0, a.lout})
       if (l.comp + (long long)(a.N - 1) * l.row + (a.ninner - 1) * l.ps >= lim) return cudaErrorInvalidValue;
     if constexpr (Narrow::NCM < Tile::NCM) {
-      if (idle_sms((a.ninner + Tile::NCM - 1) / Tile::NCM * nmem)) return epi_std<Narrow>(a, nmem, st);
+      if ((a.ninner + Tile::NCM - 1) / Tile::NCM * nmem <= 148 / 2) return epi_std<Narrow>(a, nmem, st);
     }
     return epi_std<Tile>(a, nmem, st);
   }

@@ -332,41 +332,50 @@ __global__ void __launch_bounds__(NT, MINB) k_epilogue2d(EpiArgs a) {
 #pragma unroll
     for (int g = 0; g < NB; ++g) DFT<P::RB, -1, C>::run(v[g]);
     const T k2 = T(p), kv2 = twopi * k2;  // whole wavenumber, and 2 pi times it
-    // The state values of every row first: out may be u or u0, so no load could
-    // be moved over an earlier row's store.
-    C uc[P::RB][2], wc[P::RB][2];
+    // The state values of the rows first: out may be u or u0, so no load could be moved
+    // over an earlier row's store.  Half of the rows at a time where no row is known to be
+    // dropped and all values would take more registers than there are (L = 256 FP32
+    // spilled 492 bytes, FP64 some 260 at every length; 22 solves with N = 150 and M = 256
+    // 96 -> 89 us a step, 40 FP64 ones with N = 106 and M = 192 117 -> 110).
+    constexpr int HB = STD || P::RB * Sh::CB <= 64 ? P::RB : P::RB / 2;
+    static_assert(P::RB % HB == 0);
 #pragma unroll
-    for (int b = 0; b < P::RB; ++b) {
-      if (Rt::dropped(b)) continue;
-      const int i = Rt::row(s, b, N);
-      if (!(Rt::low(b) || Rt::high(b)) && i < 0) continue;
-      const int ou = i * lu.row + p * lu.ps, ow = i * lu0.row + p * lu0.ps;
+    for (int b0 = 0; b0 < P::RB; b0 += HB) {
+      C uc[HB][2], wc[HB][2];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uc[b][c] = u[c * lu.comp + ou];
-        wc[b][c] = need_u0 ? u0[c * lu0.comp + ow] : cmk<C>(T(0), T(0));
+      for (int b = 0; b < HB; ++b) {
+        if (Rt::dropped(b0 + b)) continue;
+        const int i = Rt::row(s, b0 + b, N);
+        if (!(Rt::low(b0 + b) || Rt::high(b0 + b)) && i < 0) continue;
+        const int ou = i * lu.row + p * lu.ps, ow = i * lu0.row + p * lu0.ps;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uc[b][c] = u[c * lu.comp + ou];
+          wc[b][c] = need_u0 ? u0[c * lu0.comp + ow] : cmk<C>(T(0), T(0));
+        }
       }
-    }
 #pragma unroll
-    for (int b = 0; b < P::RB; ++b) {
-      if (Rt::dropped(b)) continue;
-      const int i = Rt::row(s, b, N);
-      if (!(Rt::low(b) || Rt::high(b)) && i < 0) continue;
-      const int oo = i * lout.row + p * lout.ps;
-      const T k1 = T(i >= N / 2 + 1 ? i - N : i), kv1 = twopi * k1;
-      const T n2 = k1 * k1 + k2 * k2;
-      const bool zero = n2 == T(0);
-      const T inv = twopi / n2;
-      const T e0 = k1 * k2, e1 = k2 * k2 - k1 * k1;
-      const C q = cmk<C>((e0 * v[0][b].x + e1 * v[1][b].x) * inv, (e0 * v[0][b].y + e1 * v[1][b].y) * inv);
-      const C Lh[2] = {cmk<C>(k2 * q.x, k2 * q.y), cmk<C>(-k1 * q.x, -k1 * q.y)};  // L / i
-      const T nu = visc_from_k2<T>(a.visc, kv1 * kv1 + kv2 * kv2, inv_k0sq);
+      for (int b = 0; b < HB; ++b) {
+        if (Rt::dropped(b0 + b)) continue;
+        const int i = Rt::row(s, b0 + b, N);
+        if (!(Rt::low(b0 + b) || Rt::high(b0 + b)) && i < 0) continue;
+        const int oo = i * lout.row + p * lout.ps;
+        const T k1 = T(i >= N / 2 + 1 ? i - N : i), kv1 = twopi * k1;
+        const T n2 = k1 * k1 + k2 * k2;
+        const bool zero = n2 == T(0);
+        const T inv = twopi / n2;
+        const T e0 = k1 * k2, e1 = k2 * k2 - k1 * k1;
+        const C v0 = v[0][b0 + b], v1 = v[1][b0 + b];
+        const C q = cmk<C>((e0 * v0.x + e1 * v1.x) * inv, (e0 * v0.y + e1 * v1.y) * inv);
+        const C Lh[2] = {cmk<C>(k2 * q.x, k2 * q.y), cmk<C>(-k1 * q.x, -k1 * q.y)};  // L / i
+        const T nu = visc_from_k2<T>(a.visc, kv1 * kv1 + kv2 * kv2, inv_k0sq);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const C x = uc[b][c], w = wc[b][c];
-        const C d = zero ? cmk<C>(T(0), T(0)) : cmk<C>(Lh[c].y + nu * x.x, nu * x.y - Lh[c].x);
-        const C t = use_u ? cmk<C>(x.x + dd * d.x, x.y + dd * d.y) : d;
-        out[c * lout.comp + oo] = cmk<C>(fma(ct, t.x - w.x, w.x), fma(ct, t.y - w.y, w.y));
+        for (int c = 0; c < 2; ++c) {
+          const C x = uc[b][c], w = wc[b][c];
+          const C d = zero ? cmk<C>(T(0), T(0)) : cmk<C>(Lh[c].y + nu * x.x, nu * x.y - Lh[c].x);
+          const C t = use_u ? cmk<C>(x.x + dd * d.x, x.y + dd * d.y) : d;
+          out[c * lout.comp + oo] = cmk<C>(fma(ct, t.x - w.x, w.x), fma(ct, t.y - w.y, w.y));
+        }
       }
     }
   }
