@@ -84,10 +84,11 @@ template <typename T, int L, int DIM> struct ZLineTile {
 // pass.  Measured (us; 2.4e8 points in FP32, 6e7 in FP64, the three stages of a
 // step averaged).  Columns: 96 as 12.8 by 16 columns 590, by 32 659; 192 as 16.12
 // 632, 12.16 760, 24.8 656; 768 as 32.24 1350, 12.8.8 1554, 16.6.8 1634; FP64 192
-// as 16.12 279, 24.8 303, 8.4.6 339.  Last pass, 2-D: 192
-// x256 as 24.8 42.8, 16.12 44.4 (16 modes 46.3); 384 x192 as 48.8 115, 24.16 131;
-// 768 x64 as 12.8.8 by 8 modes 194, by 4 221; FP64 192 as 8.3.8 475, 24.8 499, 1536
-// x1 as 16.12.8 by 2 modes 29, 12.16.8 by 1 38.
+// as 16.12 279, 24.8 303, 8.4.6 339.  32 in FP32 by 32 columns: a step of 915 3-D solves
+// with N = 18 1590, by 16 1909; shorter lengths and FP64 are slower by twice the columns.
+// Last pass, 2-D: 192 x256 as 24.8 42.8, 16.12 44.4 (16 modes 46.3); 384 x192 as 48.8
+// 115, 24.16 131; 768 x64 as 12.8.8 by 8 modes 194, by 4 221; FP64 192 as 8.3.8 475, 24.8
+// 499, 1536 x1 as 16.12.8 by 2 modes 29, 12.16.8 by 1 38.
 template <typename T, int L> struct PadTile;
 template <typename T, int L> struct Epi2Tile;
 #define AZB_LINE(Tv, Lv, A, M, B, NC_, NT_, MINB_, A2, M2, B2, NCM_, NT2, MINB2) \
@@ -105,7 +106,7 @@ AZB_LINE(float, 8, 4, 1, 2, 16, 64, 8, 4, 1, 2, 8, 32, 8)
 AZB_LINE(float, 12, 4, 1, 3, 16, 64, 8, 4, 1, 3, 8, 32, 8)
 AZB_LINE(float, 16, 4, 1, 4, 16, 64, 8, 4, 1, 4, 8, 64, 8)
 AZB_LINE(float, 24, 6, 1, 4, 16, 64, 8, 6, 1, 4, 8, 64, 8)
-AZB_LINE(float, 32, 8, 1, 4, 16, 128, 6, 8, 1, 4, 8, 64, 8)
+AZB_LINE(float, 32, 8, 1, 4, 32, 128, 6, 8, 1, 4, 8, 64, 8)
 AZB_LINE(float, 48, 8, 1, 6, 16, 128, 6, 8, 1, 6, 8, 64, 8)
 AZB_LINE(float, 64, 8, 1, 8, 16, 128, 6, 8, 1, 8, 8, 128, 4)
 AZB_LINE(float, 96, 12, 1, 8, 16, 128, 6, 12, 1, 8, 8, 96, 6)
@@ -140,8 +141,12 @@ AZB_LINE(double, 1536, 16, 12, 8, 2, 256, 2, 16, 12, 8, 2, 384, 1)
 // Tiles of 32 bytes of a row, for launches whose ordinary tiles would leave some
 // of the 148 SMs without a CTA.
 inline bool idle_sms(long long ctas) { return ctas < 148; }
+// (One FP64 2-D solve with M = 512: radices 8.8.8 instead of 32.16 here and 16.8.4
+// instead of 8.8.8 in the last pass, 66 us a step instead of 72.)
+template <typename T, int L> struct PadNarrowPlan { using P = typename PadTile<T, L>::P; };
+template <> struct PadNarrowPlan<double, 512> { using P = LinePlan<double, 512, 8, 8, 8>; };
 template <typename T, int L> struct PadTileNarrow {
-  using P = typename PadTile<T, L>::P;
+  using P = typename PadNarrowPlan<T, L>::P;
   static constexpr int NC = 32 / int(sizeof(cvec<T>));
   static constexpr int NT = kclamp((NC * (P::O > P::S ? P::O : P::S) + 31) / 32 * 32, 32, 256);
   static constexpr int MINB = 1;
@@ -149,10 +154,12 @@ template <typename T, int L> struct PadTileNarrow {
 // The last pass of 2-D solves takes them for launches of at most one ordinary tile for
 // two SMs (10 FP32 solves with N = 214 and M = 384, 140 ordinary tiles: 113 us a step with
 // narrow ones, 89 without), and with radices that leave a thread of the last stage eight
-// rows instead of sixteen (one FP32 solve: N = 150, M = 256 70 -> 60; N = 298, M = 512 90 -> 72).
+// or four rows instead of sixteen or eight (one FP32 solve: N = 150, M = 256 70 -> 60; N =
+// 298, M = 512 90 -> 72; in FP64 M = 512 see PadNarrowPlan).
 template <typename T, int L> struct Epi2NarrowPlan { using P = typename Epi2Tile<T, L>::P; };
 template <> struct Epi2NarrowPlan<float, 256> { using P = LinePlan<float, 256, 32, 1, 8>; };
 template <> struct Epi2NarrowPlan<float, 512> { using P = LinePlan<float, 512, 8, 8, 8>; };
+template <> struct Epi2NarrowPlan<double, 512> { using P = LinePlan<double, 512, 16, 8, 4>; };
 template <typename T, int L> struct Epi2TileNarrow {
   using P = typename Epi2NarrowPlan<T, L>::P;
   static constexpr int NCM = 16 / int(sizeof(cvec<T>));
