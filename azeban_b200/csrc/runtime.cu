@@ -70,7 +70,10 @@ int tuned_variant(int precision, int L, int kind) {
 // ---------------------------------------------------------------------------
 static thread_local std::string g_err;
 
+// Every failed runtime call ends here: the runtime's own copy of its error is cleared,
+// or the next launch, which asks for it, would report it again.
 static az_status fail(az_status st, const std::string& msg) {
+  if (st == AZ_ERR_CUDA || st == AZ_ERR_NOMEM) cudaGetLastError();
   g_err = msg;
   return st;
 }
