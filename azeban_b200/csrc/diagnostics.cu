@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "runtime_internal.h"
@@ -67,10 +68,10 @@ __device__ __forceinline__ void block_sum(Neu& e, Neu& w) {
 }
 
 // Partial sums over a fixed, contiguous range of modes per CTA.
-template <typename T, int DIM>
+// I: 32-bit mode indices, 64-bit ones above 2^32 modes of a component.
+template <typename T, int DIM, typename I>
 __global__ void __launch_bounds__(kDiagThreads)
-    k_diag_partials(const cvec<T>* u, unsigned N, unsigned nh, long long plane, long long member,
-                    double* parts) {
+    k_diag_partials(const cvec<T>* u, I N, I nh, long long plane, long long member, double* parts) {
   const int b = blockIdx.y;
   const long long per = (plane + kDiagParts - 1) / kDiagParts;
   const long long lo = blockIdx.x * per;
@@ -79,9 +80,9 @@ __global__ void __launch_bounds__(kDiagThreads)
   Neu e, w;
   const double twopi = 2 * 3.14159265358979323846;
   for (long long idx = lo + threadIdx.x; idx < hi; idx += kDiagThreads) {
-    const unsigned rest = unsigned(idx) / nh;  // a member has below 2^32 modes
-    const unsigned k = unsigned(idx) - rest * nh;
-    unsigned i = rest, j = 0;
+    const I rest = I(idx) / nh;
+    const I k = I(idx) - rest * nh;
+    I i = rest, j = 0;
     if (DIM == 3) {
       i = rest / N;
       j = rest - i * N;
@@ -132,13 +133,19 @@ cudaError_t diag_launch(int dim, int precision, long long N, const void* u_hat, 
   double* parts = buf;
   double* res = parts + size_t(batch) * kDiagParts * 2;
   const dim3 grid(kDiagParts, unsigned(batch));
-  if (precision == AZ_PREC_F64) {
-    if (dim == 2) k_diag_partials<double, 2><<<grid, kDiagThreads, 0, st>>>((const double2*)u_hat, unsigned(N), unsigned(nh), plane, member, parts);
-    else k_diag_partials<double, 3><<<grid, kDiagThreads, 0, st>>>((const double2*)u_hat, unsigned(N), unsigned(nh), plane, member, parts);
-  } else {
-    if (dim == 2) k_diag_partials<float, 2><<<grid, kDiagThreads, 0, st>>>((const float2*)u_hat, unsigned(N), unsigned(nh), plane, member, parts);
-    else k_diag_partials<float, 3><<<grid, kDiagThreads, 0, st>>>((const float2*)u_hat, unsigned(N), unsigned(nh), plane, member, parts);
-  }
+  const bool wide = plane > 0xffffffffLL;
+  const auto run = [&](auto t, auto d) {
+    using T = decltype(t);
+    constexpr int DIM = decltype(d)::value;
+    const auto* u = static_cast<const cvec<T>*>(u_hat);
+    using U = unsigned long long;
+    if (wide) k_diag_partials<T, DIM, U><<<grid, kDiagThreads, 0, st>>>(u, U(N), U(nh), plane, member, parts);
+    else k_diag_partials<T, DIM, unsigned><<<grid, kDiagThreads, 0, st>>>(u, unsigned(N), unsigned(nh), plane, member, parts);
+  };
+  using D2 = std::integral_constant<int, 2>;
+  using D3 = std::integral_constant<int, 3>;
+  if (precision == AZ_PREC_F64) dim == 2 ? run(0.0, D2{}) : run(0.0, D3{});
+  else dim == 2 ? run(0.0f, D2{}) : run(0.0f, D3{});
   const double Nd = dim == 2 ? double(N) * N : double(N) * N * N;
   k_diag_final<<<unsigned(batch), kDiagThreads, 0, st>>>(parts, 1.0 / (Nd * Nd), res);
   return cudaGetLastError();
