@@ -3,7 +3,7 @@
 For one workload (dimension, N, padded M, precision, batch) it runs SSP-RK3
 steps of a Simulation with every kernel variant, times each pass with the
 library's per-pass CUDA events (az_profile_*), and keeps, for each pass kind
-(column passes, epilogue pass), the fastest variant.
+that has variants there (pass_kinds), the fastest.
 Results go into a JSON tuning table that ``azeban_b200`` loads at import
 (``tuning.json`` beside this file) and applies with az_tune_set.
 
@@ -26,20 +26,23 @@ from . import _lib
 from .core import SSP_RK3, Grid, IncompressibleEuler, Simulation, make_viscosity, precision_code
 
 TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning.json")
-KIND_PASSES = {0: (0, 1, 3), 2: (4,)}  # pass ids per tuned kind
 VISC = {"type": "Smooth Cutoff", "eps": 0.05}
 
 
-# Kernel variants: the radix plan (0 std, 1 wide) of the last pass of a 3-D
-# solve (kind 2) and, at a padded length of 384, of its column passes (kind 0,
-# which is also the plan of FFT<Dim>'s strided axes).  The other passes have
-# one form per length.
+# Kernel variants: the radix plan (0 std, 1 wide).
 RUNS = (0, 1)
+# Padded lengths whose 3-D column passes have the two plans (kRegisterColumns).
+REGISTER_COLUMNS = (384,)
 
 
-def _set_all(prec: int, L: int, run: int) -> None:
-    for kind in KIND_PASSES:
-        _lib.check(_lib.lib.az_tune_set(prec, L, kind, run))
+def pass_kinds(dim: int, L: int) -> dict:
+    """Tuned kinds that the passes of a solve read, with the passes that each one times: the last pass of
+    3-D solves (kind 2) and, at some lengths, their column passes (kind 0).  The other passes have one
+    form per length.  Kinds 0 and 1 are also the plans of FFT<Dim>'s strided axes and r2c lines, which no
+    solve times."""
+    if dim != 3:
+        return {}
+    return {2: (4,), **({0: (0, 1, 3)} if L in REGISTER_COLUMNS else {})}
 
 
 def _time_passes(eq, u, reps):
@@ -63,10 +66,13 @@ def _time_passes(eq, u, reps):
 
 def autotune(dim: int, N: int, precision="f32", batch: int = 1, M: int | None = None, reps: int = 5):
     """Measures both plan variants of one workload and applies the winners;
-    returns the table entries."""
+    returns the table entries (none where no pass has variants)."""
     prec = precision_code(precision)
     g = Grid(dim, N, M)
     L = g.N_phys_pad
+    kinds = pass_kinds(dim, L)
+    if not kinds:
+        return []
     visc = make_viscosity(VISC, g)
     shape = ((batch,) if batch > 1 else ()) + g.shape_fourier(dim)
     cdt = torch.complex128 if prec == 0 else torch.complex64
@@ -74,12 +80,13 @@ def autotune(dim: int, N: int, precision="f32", batch: int = 1, M: int | None = 
     u = (torch.randn(shape, dtype=cdt, device="cuda", generator=gen) * (N ** dim) * 1e-3).contiguous()
     per_run = {}
     for run in RUNS:
-        _set_all(prec, L, run)
+        for kind in kinds:
+            _lib.check(_lib.lib.az_tune_set(prec, L, kind, run))
         eq = IncompressibleEuler(g, visc, precision, batch)
         per_run[run] = _time_passes(eq, u, reps)
         del eq
     entries = []
-    for kind, passes in KIND_PASSES.items():
+    for kind, passes in kinds.items():
         t = {run: sum(times[p] for p in passes) for run, times in per_run.items()}
         best = min(t, key=t.get)
         _lib.check(_lib.lib.az_tune_set(prec, L, kind, best))
@@ -115,6 +122,9 @@ def main(argv=None):
     ap.add_argument("--reps", type=int, default=5)
     args = ap.parse_args(argv)
     table = {}
+    if os.path.exists(args.out):  # keeps the plans that no workload times
+        with open(args.out) as f:
+            table = {(e["precision"], e["L"], e["kind"]): e for e in json.load(f)}
     for dim, N, prec, batch in WORKLOADS:
         for e in autotune(dim, N, prec, batch, reps=args.reps):
             table[(e["precision"], e["L"], e["kind"])] = e
