@@ -17,7 +17,6 @@ into status codes.  Two device-side failures are detected:
 """
 
 import contextlib
-import ctypes as ct
 
 import numpy as np
 import pytest
@@ -32,20 +31,6 @@ pytestmark = pytest.mark.gpu
 
 
 @contextlib.contextmanager
-def tuned(prec, L, kind, variant):
-    """Temporarily selects a kernel variant (bit 1 of kinds 1 and 4: the
-    bulk-copy product pass, the kernel with the bounded wait)."""
-    code = az.precision_code(prec)
-    old = ct.c_int()
-    _lib.check(_lib.lib.az_tune_get(code, L, kind, ct.byref(old)))
-    _lib.check(_lib.lib.az_tune_set(code, L, kind, variant))
-    try:
-        yield
-    finally:
-        _lib.check(_lib.lib.az_tune_set(code, L, kind, old.value))
-
-
-@contextlib.contextmanager
 def wait_limit(polls):
     old = _lib.lib.az_debug_get_wait_limit()
     _lib.check(_lib.lib.az_debug_set_wait_limit(polls))
@@ -55,8 +40,8 @@ def wait_limit(polls):
         _lib.check(_lib.lib.az_debug_set_wait_limit(old))
 
 
-def _eq(dim, N, prec, batch=1):
-    g = az.Grid(dim, N)
+def _eq(dim, N, prec, batch=1, M=None):
+    g = az.Grid(dim, N, M)
     return g, az.IncompressibleEuler(g, az.make_viscosity(VISC_CFGS["smooth"], g), prec, batch)
 
 
@@ -68,33 +53,30 @@ def _fields(dim, N, n):
 # non-finite values
 # ---------------------------------------------------------------------------
 
-@pytest.mark.parametrize("dim,N,prec,zpass", [(2, 32, "f64", False), (2, 32, "f32", True),
-                                              (3, 16, "f64", True), (3, 16, "f32", False)])
-def test_nonfinite_member_is_reported_and_isolated(dim, N, prec, zpass):
+@pytest.mark.parametrize("dim,N,prec", [(2, 32, "f64"), (2, 32, "f32"), (3, 16, "f64"), (3, 16, "f32")])
+def test_nonfinite_member_is_reported_and_isolated(dim, N, prec):
     """simulate_until returns AZ_ERR_NONFINITE when one member's state holds a
     NaN; the other members' states equal those of a clean batch bit for bit."""
     g, _ = _eq(dim, N, prec)
-    kind = 1 if dim == 3 else 4
-    with tuned(prec, g.N_phys_pad, kind, 3 if zpass else 1):
-        fields = _fields(dim, N, 4)
-        bad = [f.copy() for f in fields]
-        bad[2][0][(1,) * dim] = np.nan
-        runs = {}
-        for name, fs in (("clean", fields), ("bad", bad)):
-            _, eq = _eq(dim, N, prec, 4)
-            sim = az.Simulation(g, 0.2, az.SSP_RK3(eq), torch.stack([to_dev(f, prec) for f in fs]).contiguous())
-            if name == "bad":
-                with pytest.raises(_lib.AzebanError) as ei:
-                    sim.simulate_until(1.0)
-                assert ei.value.status == _lib.AZ_ERR_NONFINITE
-            else:
-                sim.steps(1)
-            runs[name] = (to_host(sim.u()), sim.state())
-        (clean, st_clean), (bad_u, st_bad) = runs["clean"], runs["bad"]
-        for b in (0, 1, 3):
-            assert st_bad[1][b] == 1, "the other members took their step"
-            assert np.array_equal(bad_u[b], clean[b]), f"member {b} changed by another member's NaN"
-            assert st_bad[0][b] == st_clean[0][b]
+    fields = _fields(dim, N, 4)
+    bad = [f.copy() for f in fields]
+    bad[2][0][(1,) * dim] = np.nan
+    runs = {}
+    for name, fs in (("clean", fields), ("bad", bad)):
+        _, eq = _eq(dim, N, prec, 4)
+        sim = az.Simulation(g, 0.2, az.SSP_RK3(eq), torch.stack([to_dev(f, prec) for f in fs]).contiguous())
+        if name == "bad":
+            with pytest.raises(_lib.AzebanError) as ei:
+                sim.simulate_until(1.0)
+            assert ei.value.status == _lib.AZ_ERR_NONFINITE
+        else:
+            sim.steps(1)
+        runs[name] = (to_host(sim.u()), sim.state())
+    (clean, st_clean), (bad_u, st_bad) = runs["clean"], runs["bad"]
+    for b in (0, 1, 3):
+        assert st_bad[1][b] == 1, "the other members took their step"
+        assert np.array_equal(bad_u[b], clean[b]), f"member {b} changed by another member's NaN"
+        assert st_bad[0][b] == st_clean[0][b]
 
 
 @pytest.mark.parametrize("dim,N", [(2, 16), (3, 8)])
@@ -124,33 +106,32 @@ def test_nonfinite_rk3_and_dt(dim, N):
 # bounded waits that run out
 # ---------------------------------------------------------------------------
 
-@pytest.mark.parametrize("dim,N,prec", [(3, 32, "f32"), (3, 16, "f64"), (2, 64, "f32")])
-def test_bounded_wait_timeout_is_reported(dim, N, prec):
-    g = az.Grid(dim, N)
-    kind = 1 if dim == 3 else 4
+@pytest.mark.parametrize("dim,N,M,M_oracle,prec", [(3, 32, 48, 48, "f32"), (3, 16, 24, 24, "f64"), (2, 64, 96, 96, "f32"),
+                                                   (3, 16, 384, 36, "f32"), (3, 16, 384, 36, "f64")])
+def test_bounded_wait_timeout_is_reported(dim, N, M, M_oracle, prec):
+    """In k_zline and, in 3-D at M = 384, k_zfused (whose right-hand side is that of a smaller M)."""
     u = random_field_hat(dim, N, seed=31)
-    og = ora.Grid(dim, N)
+    og = ora.Grid(dim, N, M_oracle)
     ref = ora.IncompressibleEuler(og, ora.make_viscosity(VISC_CFGS["smooth"], og)).dudt(u)
-    with tuned(prec, g.N_phys_pad, kind, 3):
-        _, eq = _eq(dim, N, prec)  # kernel variants are fixed when the equation is created
-        d_u = to_dev(u, prec)
-        out = torch.empty_like(d_u)
-        with wait_limit(0):
-            eq.dudt(out, d_u)
-            with pytest.raises(_lib.AzebanError) as ei:
-                eq.dt(0.2)
-            assert ei.value.status == _lib.AZ_ERR_TIMEOUT
-            # a simulation created (and its step graph captured) under the limit
-            sim = az.Simulation(g, 0.2, az.SSP_RK3(eq), d_u)
-            with pytest.raises(_lib.AzebanError) as ei:
-                sim.simulate_until(0.01)
-            assert ei.value.status == _lib.AZ_ERR_TIMEOUT
-            del sim
-        torch.cuda.synchronize()
-        # the context is intact: the next right-hand side is right again
+    g, eq = _eq(dim, N, prec, M=M)
+    d_u = to_dev(u, prec)
+    out = torch.empty_like(d_u)
+    with wait_limit(0):
         eq.dudt(out, d_u)
-        assert eq.dt(0.2) > 0
-        assert rel_l2(to_host(out), ref) <= (1e-12 if prec == "f64" else 1e-5)
+        with pytest.raises(_lib.AzebanError) as ei:
+            eq.dt(0.2)
+        assert ei.value.status == _lib.AZ_ERR_TIMEOUT
+        # a simulation created (and its step graph captured) under the limit
+        sim = az.Simulation(g, 0.2, az.SSP_RK3(eq), d_u)
+        with pytest.raises(_lib.AzebanError) as ei:
+            sim.simulate_until(0.01)
+        assert ei.value.status == _lib.AZ_ERR_TIMEOUT
+        del sim
+    torch.cuda.synchronize()
+    # the context is intact: the next right-hand side is right again
+    eq.dudt(out, d_u)
+    assert eq.dt(0.2) > 0
+    assert rel_l2(to_host(out), ref) <= (1e-12 if prec == "f64" else 1e-5)
 
 
 def test_wait_limit_rejects_negative():

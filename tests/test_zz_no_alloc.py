@@ -130,18 +130,13 @@ def test_noalloc_status_reports_device_failures():
     stream = torch.cuda.current_stream().cuda_stream or None
     u = to_dev(random_field_hat(dim, N, seed=5), prec)
     out = torch.empty_like(u)
-    code = az.precision_code(prec)
-    old_v = ct.c_int()
-    _lib.check(_lib.lib.az_tune_get(code, g.N_phys_pad, 1, ct.byref(old_v)))
     old_polls = _lib.lib.az_debug_get_wait_limit()
     try:
-        _lib.check(_lib.lib.az_tune_set(code, g.N_phys_pad, 1, 3))  # the bulk-copy product pass
         _lib.check(_lib.lib.az_debug_set_wait_limit(0))
         _lib.check(_noalloc(dim, N, g.N_phys_pad, prec, visc, out, u))
         assert _lib.lib.az_euler_noalloc_status(stream) == _lib.AZ_ERR_TIMEOUT
     finally:
         _lib.check(_lib.lib.az_debug_set_wait_limit(old_polls))
-        _lib.check(_lib.lib.az_tune_set(code, g.N_phys_pad, 1, old_v.value))
     bad = u.clone()
     bad[0, 1, 1, 1] = float("nan")
     _lib.check(_noalloc(dim, N, g.N_phys_pad, prec, visc, out, bad))
