@@ -225,14 +225,9 @@ template <typename T, typename P, int NCM> struct Epi2Shape {
   static constexpr int STR = line_stride(P::RB * COLS, W * NCM, CB);
   static constexpr int TW = (P::NTW + W - 1) / W * W;
   static constexpr size_t BYTES = size_t(TW + P::S * STR) * CB;
-  // Place of component c of mode pl in a row: component groups of W apart, the
-  // modes of a group contiguous (the last stage's lanes), exchanged by an XOR
-  // that puts the groups of neighbouring modes (the first stage's lanes) in
-  // different banks.
-  static __host__ __device__ constexpr int place(int c, int pl) {
-    const int g = c / W, few = 128 / (CB * NB);  // modes whose components fill a wavefront
-    return g * (W * NCM) + (pl ^ (NCM >= few * (NB / W) ? g * few : (g * W * NCM * CB / 128 * few) & (NCM - 1))) * W + c % W;
-  }
+  // Place of component c of mode pl in a row: groups of the W components that a thread
+  // reads at once, the modes of a group contiguous (the last stage's lanes).
+  static __host__ __device__ constexpr int place(int c, int pl) { return c / W * (W * NCM) + pl * W + c % W; }
 };
 
 // Last pass of a 2-D right-hand side: forward along x of B11 - B22 and B12 (a

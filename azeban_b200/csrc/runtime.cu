@@ -49,6 +49,8 @@ static const int kLengths[] = {
 // Tuning table: plan variant per (precision, length, pass kind).  Defaults:
 // FP32 uses the wide plans (fewer exchanges), FP64 the register-lean ones.
 // AZ_PLAN_VARIANT="c,r,e" overrides every entry; az_tune_set overrides one.
+// Only bit 0 of kinds 0 (k_cols), 1 (r2c lines of FFT<Dim>) and 2 (3-D last pass)
+// picks a kernel; the other bits and kinds 3 to 5 are taken and given back.
 // ---------------------------------------------------------------------------
 static std::mutex g_tune_mutex;
 static std::map<std::tuple<int, int, int>, int> g_tune;
@@ -288,9 +290,8 @@ az_status az_euler_create(const az_euler_desc* d, az_euler* out) {
   e->eps_visc = d->visc.type == AZ_VISC_NONE ? 0.0 : d->visc.eps;
   e->ks = ks;
   e->csize = d->precision == 0 ? 16 : 8;
-  const int kbase = e->dim == 2 ? 3 : 0;
-  e->v_cols = tuned_variant(e->prec, int(e->M), kbase + 0);
-  e->v_epi = tuned_variant(e->prec, int(e->M), kbase + 2);
+  e->v_cols = tuned_variant(e->prec, int(e->M), 0);
+  e->v_epi = tuned_variant(e->prec, int(e->M), 2);
   euler_layout(e);
   e->state_elems = e->state_mem * e->batch;
   size_t off[3];

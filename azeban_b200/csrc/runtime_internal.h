@@ -36,7 +36,7 @@ struct az_euler_s {
   double norm;
   double Md;
   bool prof = true;  // false: never record per-pass timing events
-  int v_cols = 0, v_epi = 0;  // plan variants of the column and epilogue passes
+  int v_cols = 0, v_epi = 0;  // plan variants of k_cols and of the 3-D last pass
   double* diag = nullptr;  // partial sums of the energy / enstrophy reduction
 };
 
