@@ -2,14 +2,18 @@
 // real lines share one complex transform, line a in the real part, line b in the
 // imaginary part.
 //
-// c2r: the stages, places and twiddles are k_zline's inverse with one component
-// (zline.cuh): the first stage reads the half spectra, the last one writes the
-// lines, and lanes run along the lines in both.  256^3 x 3 FP64: 160 us against
-// 249 us when lines were staged in shared memory on the way in and out (124 us
-// for the bytes alone at the copy bandwidth).
-// r2c keeps the earlier form: the same rework took it from 196 to 130 us there,
-// but moved single modes of a 256^3 vortex's spectrum by up to 1.3e-12 of its
-// root mean square, close to all that a change of version may (1.5e-12).
+// c2r: the stages, places, twiddles and radices are those of k_zline's inverse in 2-D
+// with one component (zline.cuh): the first stage reads the half spectra, the last one
+// writes the lines, and lanes run along the lines in both.  256^3 x 3 FP64: 169 us
+// against 249 us when lines were staged in shared memory on the way in and out (124 us
+// for the bytes alone at the copy bandwidth).  Two stages of larger radices (8.24, 16.16,
+// 16.24) are slower or the same: whole backward transforms (us, two stages -> these)
+// 192^3 x3 FP64 265 -> 244, 256^3 x3 FP64 469 -> 478, 384^3 x3 FP64 1865 -> 1678, FP32 868
+// -> 849; two fields of 256^2 in FP64 12.2 -> 9.9.
+// r2c keeps the earlier form.  In this structure it takes 130 us instead of 196 there
+// and adds in another order, which moves single modes of a 256^3 Taylor-Green vortex's
+// spectrum, beside those that hold its energy, by up to 1.3e-12 of the root mean square
+// of the others; the tolerance of that transform in perf/cases.py leaves no room for it.
 //
 // Reference: src/azeban/cuda/operations/cufft.cpp:133-149.
 #pragma once
@@ -27,15 +31,8 @@ struct RealRowArgs {
   long long in_line, out_line;  // in elements of the respective type
 };
 
-// The radices of the 2-D product pass's inverse, but at 192, 256 and 384 the
-// two-stage plans these lines have always had.
-template <typename T, int L> struct RowPlan : ZPlan<T, L, 2> {};
-template <typename T> struct RowPlan<T, 192> { static constexpr int R1 = 8, R2 = 1, RM = 24; };
-template <typename T> struct RowPlan<T, 256> { static constexpr int R1 = 16, R2 = 1, RM = 16; };
-template <typename T> struct RowPlan<T, 384> { static constexpr int R1 = 16, R2 = 1, RM = 24; };
-
 template <typename T, int L> struct RowShape {
-  using P = RowPlan<T, L>;
+  using P = ZPlan<T, L, 2>;
   static constexpr int CB = int(sizeof(cvec<T>));
   static constexpr int S = L / P::RM;
   static constexpr int NLP = S >= 128 ? 1 : 128 / S;  // line pairs of a CTA
