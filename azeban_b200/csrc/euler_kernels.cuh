@@ -60,7 +60,7 @@ struct ColArgs {
   int clear_max;  // nonzero: the first pass; reset the member's CFL accumulator
   int begin;      // StepBegin, with its max_dt
   double max_dt;
-  int pdl;        // programmatic dependent launch
+  int pdl;        // to launch_pass: may be a programmatic dependent; to the kernel: is one
   int in_ci;      // input component interleave: column p reads component p % in_ci
                   // at in_comp stride, position p / in_ci (1: plain columns)
   // Grouped columns (grp > 0): column p is entry q = p % grp of group
@@ -177,7 +177,7 @@ struct EpiArgs {
   Ctrl* ctrl;
   double C, Md;  // MODE_RK1: dt = min(C / (N u_max), max_dt), u_max = max / M^d, is set here
   int end_step;  // the last pass of a step inside simulate_until: time += dt
-  int pdl;       // programmatic dependent launch
+  int pdl;       // to launch_pass: may be a programmatic dependent; to the kernel: is one
   // > 0: B's modes are grouped, nh per group with a group stride of b_grp
   // elements (the padded rows of B2 [M][N][b_grp]); 0: contiguous modes.
   long long b_grp;

@@ -18,8 +18,8 @@
 // stages, two barriers per exchange) a thread holds one butterfly at a time, which
 // leaves registers for radices up to 32, two stages up to L = 1024 and more
 // loads in flight.  Measured (us, before -> after): 512^3 FP32 inverse y 1622 ->
-// 1331, forward y (5 components) 2530 -> 2243; 128^3 FP64 53 -> 43 and 71 -> 62;
-// 2-D last pass 128^2 x256 FP32 54 -> 43.
+// 1336, forward y 2992 -> 2642; 128^3 FP64 54 -> 42 and 81 -> 71; 2-D last pass 128^2
+// x256 FP32 54 -> 43.
 #pragma once
 
 #include "euler_kernels.cuh"

@@ -387,8 +387,8 @@ static StateLayout state_layout(az_euler e, bool inner) {
 // begin, max_dt: what the first pass does to the control blocks (StepBegin).
 // MODE_RK1: the step size dt = min(C/(N u_max), max_dt) is set on the way.
 // end_step: the last pass also moves the members' clocks.
-// Passes after the first, and the first of a later stage, are programmatic
-// dependents of the kernel before them.
+// Passes after the first, and the first of a later stage, may be programmatic
+// dependents of the kernel before them (launch_pass).
 // u_inner / u0_inner / out_inner: the array is in the component-innermost
 // layout (else planar).
 static az_status rhs(az_euler e, const void* u, bool u_inner, const void* u0, bool u0_inner, void* out,

@@ -118,7 +118,7 @@ struct ZArgs {
   double norm;       // 1 / (N^{d/2} M^{d/2})
   Ctrl* ctrl;
   int wait_polls;    // limit of the wait for the chunk's bulk copy (kWaitPolls)
-  int pdl;           // programmatic dependent launch
+  int pdl;           // to launch_pass: may be a programmatic dependent; to the kernel: is one
 };
 
 // Product c of the velocities u: 11, 12, 22 in 2-D; 11, 21, 22, 31, 32, 33 in 3-D

@@ -293,7 +293,7 @@ def run_ours(args, rank, world, local):
     nl = (ct.c_longlong * 5)()
     _lib.check(_lib.lib.az_profile_read(ms, by, nl, 5))
     pass_names = ["inv_x_pad", "inv_y_pad", "z_product", "fwd_y_trunc", "fwd_x_epilogue"]
-    product_kernel = "k_zfused" if g.N_phys_pad == 384 else "k_zline"  # six products at 384
+    product_kernel = "k_zfused" if g.N_phys_pad == 384 else "k_zline"  # kRegisterColumns
     kernel_keys = ["k_cols_pad_inv_x", "k_cols_pad_inv_y", product_kernel,
                    "k_cols_trunc_fwd", "k_fwd_epilogue"]
     peak, peak_kind = measured_peak_hbm()
